@@ -81,10 +81,24 @@ int ensure_device(int* num_sms) {
     }
     g_dev[dev].num_sms = prop.multiProcessorCount;
     CUDA_TRY(configure_grouped_gemm());
-    CUDA_TRY(configure_decode_gemm());
+    CUDA_TRY(configure_stream_gemm());
     g_dev[dev].ready = true;
   }
   *num_sms = g_dev[dev].num_sms;
+  return B200MOE_OK;
+}
+
+// Bytes in boxes with 128-byte swizzle.
+int encode_tmap(CUtensorMap* map, const void* base, uint32_t rank, const cuuint64_t* dims, const cuuint64_t* strides,
+                const cuuint32_t* box) {
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, rank, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    snprintf(g_cuda_error, sizeof(g_cuda_error), "cuTensorMapEncodeTiled (%uD) failed with CUresult %d", rank, (int)r);
+    return B200MOE_ERR_CUDA;
+  }
   return B200MOE_OK;
 }
 
@@ -93,15 +107,7 @@ int make_tmap(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k, uin
   cuuint64_t dims[2] = {k, rows};
   cuuint64_t strides[1] = {pitch};
   cuuint32_t box[2] = {(cuuint32_t)kBlockK, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    snprintf(g_cuda_error, sizeof(g_cuda_error), "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
-    return B200MOE_ERR_CUDA;
-  }
-  return B200MOE_OK;
+  return encode_tmap(map, base, 2, dims, strides, box);
 }
 
 // GEMM1 weights [e_local][2*inter][k] seen as planes: plane 2e holds expert e's gate rows, plane
@@ -114,26 +120,32 @@ int make_tmap_gate_up(CUtensorMap* map, const void* base, uint64_t e_local, uint
   cuuint64_t dims[3] = {k, inter, 2 * e_local};
   cuuint64_t strides[2] = {k, inter * k};
   cuuint32_t box[3] = {(cuuint32_t)kBlockK, box_rows, 2};
-  cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) {
-    snprintf(g_cuda_error, sizeof(g_cuda_error), "cuTensorMapEncodeTiled (3D) failed with CUresult %d", (int)r);
-    return B200MOE_ERR_CUDA;
-  }
-  return B200MOE_OK;
+  return encode_tmap(map, base, 3, dims, strides, box);
+}
+
+// The same with the K blocks as a dimension of their own (128 bytes apart), so that one box brings `box_kb` K blocks, each
+// as a swizzled tile behind the other: rows x K, and the gate and up planes of GEMM1.
+int make_tmap_kblocks(CUtensorMap* map, const void* base, uint64_t rows, uint64_t k, uint32_t box_rows, uint32_t box_kb) {
+  cuuint64_t dims[3] = {(cuuint64_t)kBlockK, rows, k / kBlockK};
+  cuuint64_t strides[2] = {k, (cuuint64_t)kBlockK};
+  cuuint32_t box[3] = {(cuuint32_t)kBlockK, box_rows, box_kb};
+  return encode_tmap(map, base, 3, dims, strides, box);
+}
+int make_tmap_gate_up_kblocks(CUtensorMap* map, const void* base, uint64_t e_local, uint64_t inter, uint64_t k,
+                              uint32_t box_rows, uint32_t box_kb) {
+  cuuint64_t dims[4] = {(cuuint64_t)kBlockK, inter, 2 * e_local, k / kBlockK};
+  cuuint64_t strides[3] = {k, inter * k, (cuuint64_t)kBlockK};
+  cuuint32_t box[4] = {(cuuint32_t)kBlockK, box_rows, 2, box_kb};
+  return encode_tmap(map, base, 4, dims, strides, box);
 }
 
 uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
 constexpr int kDirectRowsMaxTokens = 8;   // largest call whose decode GEMM1 reads the caller's rows in place
 
-// Decode-size calls (up to 16 tokens) take the swapped-operand kernels (B200MOE_DECODE=0 turns them off;
-// B200MOE_DECODE=64 extends them to 64 tokens, where the 128-row tiles currently measure faster).  Their
-// per-warp scale panels hold a bounded number of K blocks; larger shapes take the grouped kernels.
-// Returns the token tile of the decode kernels, or 0 for the grouped kernels.
-int decode_tile(int T, int hidden, int inter) {
+// Decode-size calls (up to 16 tokens) requantise inside GEMM1 (B200MOE_DECODE=0 turns that off, B200MOE_DECODE=64
+// extends it to 64 tokens).  Returns the token tile of the streaming kernels for such a call, or 0.
+int decode_tile(int T) {
   static const bool decode_on = [] {
     const char* v = getenv("B200MOE_DECODE");
     return !(v && v[0] == '0');
@@ -142,8 +154,23 @@ int decode_tile(int T, int hidden, int inter) {
     const char* v = getenv("B200MOE_DECODE");
     return (v && v[0] == '6') ? 64 : 16;
   }();
-  const bool fits = hidden / kBlockK <= decode_gemm_max_kblocks() && inter / kBlockK <= decode_gemm_max_kblocks();
-  return (decode_on && fits && T <= decode_max_t) ? (T <= 16 ? 16 : 64) : 0;
+  return (decode_on && T <= decode_max_t) ? (T <= 16 ? 16 : 64) : 0;
+}
+
+// Calls above the decode sizes and up to this many tokens take the weight-streaming GEMMs if few enough experts are local.
+// The 128 x 256 tiles of the grouped kernel come in whole waves of SMs: with some ten to twenty active experts (two waves
+// of GEMM1 items) the second is mostly idle, with more than a hundred it does not matter and the grouped kernel's larger
+// boxes win (56 tokens, 32 experts: 131 -> 115 us with 10 active, 166 -> 163 with 18; 64 tokens, 256 experts: 915 against
+// 945 us).  B200MOE_STREAM=0: never.
+constexpr int kStreamMaxTokens = 64;
+constexpr int kStreamMaxExperts = 64;
+// Returns the most token rows of a tile (an expert of a call of at most 64 tokens has no more), or 0 for the grouped kernels.
+int stream_tile(int T, int e_local) {
+  static const bool on = [] {
+    const char* v = getenv("B200MOE_STREAM");
+    return !(v && v[0] == '0');
+  }();
+  return on && T <= kStreamMaxTokens && e_local <= kStreamMaxExperts ? 64 : 0;
 }
 
 int shape_ok(int T, int e_local, int hidden, int inter) {
@@ -171,7 +198,7 @@ void compute_layout(int T, int e_local, int hidden, int inter, b200moe_ws_layout
   auto take = [&](uint64_t bytes) { uint64_t o = off; off = align_up(off + bytes, 256); return o; };
   L->status = take(16 * 4);
   L->meta = take(8 * 4);
-  L->splitk_count = take(2 * kSplitKSlots * 4);   // inside the range that clear_counters() zeroes
+  L->splitk_count = take(2 * kStreamMaxCtas * 4);   // inside the range that clear_counters() zeroes
   L->tile_done = take((uint64_t)L->max_tiles * 4);   // likewise
   L->chunk_counts = take((uint64_t)n_chunks * e_local * 4);
   L->chunk_base = take((uint64_t)n_chunks * e_local * 4);
@@ -190,7 +217,8 @@ void compute_layout(int T, int e_local, int hidden, int inter, b200moe_ws_layout
   L->topk_ids = take((uint64_t)(T > 0 ? T : 1) * kTopK * 4);
   L->topk_w = take((uint64_t)(T > 0 ? T : 1) * kTopK * 4);
   L->trace = take(2 * 8 * 64 * 8);   // B200MOE_PROF: absolute cycle stamps of CTA 0's first 64 K blocks
-  L->splitk_scratch = take((uint64_t)kSplitKSlots * kSplitKMax * 16 * 128 * 4);   // 2 MiB
+  // two cut tiles per CTA of the streaming GEMMs: 2.5 MiB at decode sizes, 10 MiB (64 token rows) above
+  L->splitk_scratch = take((uint64_t)2 * kStreamMaxCtas * (T <= 16 ? 16 : 64) * 128 * 4);
   L->ep_segments = take(256);   // RowSegments at +0, int32 row count at +192 (b200moe_ep_local_experts)
   L->total_bytes = off;
 }
@@ -203,6 +231,22 @@ int bind_workspace(int T, int e_local, int hidden, int inter, void* workspace, s
   compute_layout(T, e_local, hidden, inter, &ws->L);
   if (bytes < ws->L.total_bytes) return B200MOE_ERR_WORKSPACE_TOO_SMALL;
   ws->base = reinterpret_cast<uint8_t*>(workspace);
+  return B200MOE_OK;
+}
+
+// K blocks of a box of the streaming kernels
+uint32_t group_kblocks(int k) { return k / kBlockK < kStreamGroup ? k / kBlockK : kStreamGroup; }
+
+// What the streaming kernels take beside a GEMM's ordinary arguments: the packed rows ([m_cap][k] at `rows_off`) in boxes
+// of 16, 32 and 64 rows.
+int make_stream_params(StreamParams* sp, const GemmParams& g, const Workspace& ws, uint64_t rows_off, int k) {
+  sp->g = g;
+  sp->expert_row0 = ws.at<int>(ws.L.expert_row0);
+  for (int c = 0; c < 3; ++c) {
+    const int rc = make_tmap_kblocks(&sp->tmap_tok[c], ws.base + rows_off, (uint64_t)ws.L.m_cap, (uint64_t)k, 16u << c,
+                                     group_kblocks(k));
+    if (rc != B200MOE_OK) return rc;
+  }
   return B200MOE_OK;
 }
 
@@ -347,7 +391,10 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   if ((rc = ensure_device(&num_sms)) != B200MOE_OK) return rc;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 
-  const int nt = decode_tile(T, hidden, inter);
+  const bool fits = stream_gemm_fits(hidden / kBlockK, ws.L.max_tiles, num_sms) &&
+                    stream_gemm_fits(inter / kBlockK, ws.L.max_tiles, num_sms);
+  const int nt = fits ? decode_tile(T) : 0;                      // > 0: GEMM1 also requantises
+  const int slab_nt = nt ? nt : (fits ? stream_tile(T, e_local) : 0);     // > 0: the streaming kernels (slabs of 128 weight rows)
   // A call of at most 8 tokens that the one-block front kernel routed and placed runs no gather pass: its GEMM1
   // fetches the token rows and their scales where the caller keeps them (and zeroes the output rows).  Measured
   // with inputs cold in HBM: -4 us at 1 token, -2 at 4, but +2..4 at 16 tokens with 4 rows (56 separate 128-byte
@@ -366,13 +413,14 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
         B200MOE_OK)
       return rc;
   } else if ((rc = make_tmap(&g1.tmap_a, ws.base + ws.L.a_packed, (uint64_t)ws.L.m_cap, (uint64_t)hidden,
-                             (uint64_t)hidden, nt ? nt : kTileM)) != B200MOE_OK) {
+                             (uint64_t)hidden, kTileM)) != B200MOE_OK) {
     return rc;
   }
-  // one box = 128 gate rows + the matching 128 up rows (decode kernels: 64 + 64)
-  if ((rc = make_tmap_gate_up(&g1.tmap_b, w1, (uint64_t)e_local, (uint64_t)inter, (uint64_t)hidden, nt ? 64 : 128)) !=
-      B200MOE_OK)
-    return rc;
+  // one box = 128 gate rows + the matching 128 up rows (streaming kernels: 64 + 64, a group of K blocks)
+  rc = slab_nt ? make_tmap_gate_up_kblocks(&g1.tmap_b, w1, (uint64_t)e_local, (uint64_t)inter, (uint64_t)hidden, 64,
+                                           group_kblocks(hidden))
+               : make_tmap_gate_up(&g1.tmap_b, w1, (uint64_t)e_local, (uint64_t)inter, (uint64_t)hidden, 128);
+  if (rc != B200MOE_OK) return rc;
   g1.meta = ws.at<int>(ws.L.meta);
   g1.tile_expert = ws.at<int>(ws.L.tile_expert);
   g1.row_token = ws.at<int>(ws.L.row_token);
@@ -381,13 +429,13 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g1.m_cap = ws.L.m_cap;
   g1.n_per_expert = 2 * inter;
   g1.kblocks = hidden / kBlockK;
-  g1.n_tiles = nt ? inter / 64 : inter / 128;
+  g1.n_tiles = slab_nt ? inter / 64 : inter / 128;
   g1.expert_count = ws.at<int>(ws.L.expert_count);
   g1.inter = inter;
   g1.hidden = hidden;
   g1.act = ws.at<__half>(ws.L.act);
   g1.row_amax = ws.at<unsigned>(ws.L.row_amax);
-  g1.tile_done = ws.at<int>(ws.L.tile_done);
+  g1.tile_done = nt ? ws.at<int>(ws.L.tile_done) : nullptr;
   g1.act_q_out = ws.at<uint8_t>(ws.L.act_q);
   g1.row_scale_out = ws.at<float>(ws.L.row_scale);
   g1.direct_a = direct_a ? 1 : 0;
@@ -408,7 +456,14 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g1.trace = prof_on ? ws.at<unsigned long long>(ws.L.trace) : nullptr;
   if (g_prof_start) CUDA_TRY(cudaEventRecord(g_prof_start, st));
   {
-    cudaError_t le = nt ? launch_decode_gemm(1, nt, g1, num_sms, st) : launch_grouped_gemm(1, g1, num_sms, st);
+    cudaError_t le;
+    if (slab_nt) {
+      StreamParams s1;
+      if ((rc = make_stream_params(&s1, g1, ws, ws.L.a_packed, hidden)) != B200MOE_OK) return rc;
+      le = launch_stream_gemm(1, slab_nt, s1, ws.L.max_tiles, num_sms, st);
+    } else {
+      le = launch_grouped_gemm(1, g1, num_sms, st);
+    }
     cudaEvent_t stop = g_prof_stop;
     g_prof_start = g_prof_stop = nullptr;   // one shot, whatever happens next
     if (le != cudaSuccess) return cuda_fail(le, "GEMM1 launch");
@@ -422,11 +477,12 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   GemmParams g2;
   memset(&g2, 0, sizeof(g2));
   if ((rc = make_tmap(&g2.tmap_a, ws.base + ws.L.act_q, (uint64_t)ws.L.m_cap, (uint64_t)inter, (uint64_t)inter,
-                      nt ? nt : kTileM)) != B200MOE_OK)
+                      kTileM)) != B200MOE_OK)
     return rc;
-  if ((rc = make_tmap(&g2.tmap_b, w2, (uint64_t)e_local * hidden, (uint64_t)inter, (uint64_t)inter,
-                      nt ? 128 : 256)) != B200MOE_OK)   // the whole B tile (decode: the 128-row slab) in one box
-    return rc;
+  // the whole B tile (or the 128-row slab of a group of K blocks) in one box
+  rc = slab_nt ? make_tmap_kblocks(&g2.tmap_b, w2, (uint64_t)e_local * hidden, (uint64_t)inter, 128, group_kblocks(inter))
+               : make_tmap(&g2.tmap_b, w2, (uint64_t)e_local * hidden, (uint64_t)inter, (uint64_t)inter, 256);
+  if (rc != B200MOE_OK) return rc;
   g2.meta = g1.meta;
   g2.tile_expert = g1.tile_expert;
   g2.row_token = g1.row_token;
@@ -434,7 +490,7 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g2.m_cap = ws.L.m_cap;
   g2.n_per_expert = hidden;
   g2.kblocks = inter / kBlockK;
-  g2.n_tiles = nt ? hidden / 128 : hidden / 256;
+  g2.n_tiles = slab_nt ? hidden / 128 : hidden / 256;
   g2.expert_count = g1.expert_count;
   g2.inter = inter;
   g2.hidden = hidden;
@@ -445,11 +501,16 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g2.status = g1.status;
   g2.status_mirror = g1.status_mirror;
   g2.splitk_scratch = g1.splitk_scratch;
-  g2.splitk_count = g1.splitk_count + kSplitKSlots;
+  g2.splitk_count = g1.splitk_count + kStreamMaxCtas;
   g2.prof = prof_on ? ws.at<unsigned long long>(ws.L.meta + 136) : nullptr;
   g2.trace = prof_on ? ws.at<unsigned long long>(ws.L.trace) + 8 * 64 : nullptr;
-  if (nt) CUDA_TRY(launch_decode_gemm(2, nt, g2, num_sms, st));
-  else CUDA_TRY(launch_grouped_gemm(2, g2, num_sms, st));
+  if (slab_nt) {
+    StreamParams s2;
+    if ((rc = make_stream_params(&s2, g2, ws, ws.L.act_q, inter)) != B200MOE_OK) return rc;
+    CUDA_TRY(launch_stream_gemm(2, slab_nt, s2, ws.L.max_tiles, num_sms, st));
+  } else {
+    CUDA_TRY(launch_grouped_gemm(2, g2, num_sms, st));
+  }
 
   // nothing follows GEMM2: its epilogue added every packed row into its token's output row
   return B200MOE_OK;

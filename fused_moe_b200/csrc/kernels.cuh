@@ -49,10 +49,10 @@ cudaError_t launch_route_place_small(const Workspace& ws, const void* logits, in
                                      int bias_dtype, int T, float rsf, int local_off, int e_local, int pad_rows,
                                      cudaStream_t stream);
 
-// Decode GEMMs split the K range of a weight slab over up to kSplitKMax CTAs when a call has at
-// most kSplitKSlots (expert tile, slab) items, i.e. fewer than half of the SMs would stream weights.
-constexpr int kSplitKSlots = 64;
-constexpr int kSplitKMax = 4;
+// The weight-streaming GEMMs (gemm_stream.cu) run on at most this many CTAs, each of which may leave two cut tiles of
+// 128 weight rows x nt token rows of partial sums.
+constexpr int kStreamMaxCtas = 160;
+constexpr int kStreamGroup = 2;   // K blocks that travel and are handed over together
 
 // Arguments of the two grouped GEMMs.  `tmap_a` covers the packed rows [m_cap][K],
 // `tmap_b` the weights viewed as [e_local * N][K]; both e4m3, 128-byte swizzled boxes.
@@ -62,7 +62,7 @@ struct GemmParams {
   const int* meta;          // [0] = number of 128-row M tiles
   const int* tile_expert;   // expert of each M tile
   const int* row_token;     // token of each packed row, -1 for padding
-  const int* expert_count;  // rows per local expert (decode kernel)
+  const int* expert_count;  // rows per local expert (streaming kernel)
   const float* a_scale;     // GEMM1: [K/128][m_cap] activation scales
   const float* b_scale;     // [e_local][N/128][K/128] weight scales
   int m_cap;
@@ -73,7 +73,7 @@ struct GemmParams {
   int hidden;
   __half* act;              // GEMM1 out: [m_cap][inter] fp16
   unsigned* row_amax;       // GEMM1 out: bits of max |act| per row
-  int* tile_done;           // decode GEMM1: slabs of each expert tile whose activations are stored (zero at call start)
+  int* tile_done;           // decode GEMM1 (else null): slabs of each expert tile whose activations are stored (zero at call start)
   uint8_t* act_q_out;       // decode GEMM1 out (the CTA that stores an expert's last slab): [m_cap][inter] e4m3
   float* row_scale_out;     // decode GEMM1 out (same CTA): requantisation scale per row
   const float* row_scale;   // GEMM2 in: requantisation scale per row
@@ -88,8 +88,8 @@ struct GemmParams {
   long long hs_stride_t, hs_stride_kb;
   int* status;
   int* status_mirror;       // optional host-mapped int32[4]: receives the status word when a CTA gives up on a wait
-  float* splitk_scratch;    // decode GEMMs: [kSplitKSlots][kSplitKMax][16][128] partial sums
-  int* splitk_count;        // decode GEMMs: arrivals per weight slab, zero at kernel start and end
+  float* splitk_scratch;    // streaming GEMMs: [2 per CTA][nt][128] partial sums of cut tiles
+  int* splitk_count;        // streaming GEMMs: arrivals at the tile that a CTA begins and others finish, zero at kernel start and end
   unsigned long long* prof;   // optional cycle counters of CTA 0 (null: off)
   unsigned long long* trace;  // optional [64][8] absolute cycle stamps of CTA 0's first K blocks
 };
@@ -99,10 +99,17 @@ cudaError_t launch_grouped_gemm(int mode, const GemmParams& p, int num_sms, cuda
 cudaError_t configure_grouped_gemm();   // opt-in shared memory sizes, once per process and device
 int grouped_gemm_max_kblocks();         // largest K / 128 the kernels' scale panels hold
 
-// Decode sizes (T <= nt, nt 16 or 64): operands swapped, weights on the MMA's M side (gemm_decode.cu).
-cudaError_t launch_decode_gemm(int mode, int nt, const GemmParams& p, int num_sms, cudaStream_t stream);
-cudaError_t configure_decode_gemm();
-int decode_gemm_max_kblocks();          // largest K / 128 its per-warp scale panels hold
+// Few rows per expert (gemm_stream.cu): operands swapped (weights on the MMA's M side), the call's (tile, K block) units
+// in one contiguous range per CTA.  nt 16 or 64: most token rows of a tile.
+struct StreamParams {
+  GemmParams g;               // tmap_b: boxes of kStreamGroup K blocks x 64 gate + 64 up rows (GEMM1), 128 rows (GEMM2); tmap_a:
+                              // direct_a only (one row, one K block)
+  CUtensorMap tmap_tok[3];    // the packed rows in boxes of kStreamGroup K blocks x 16, 32, 64 rows
+  const int* expert_row0;
+};
+cudaError_t launch_stream_gemm(int mode, int nt, const StreamParams& p, int max_tiles, int num_sms, cudaStream_t stream);
+cudaError_t configure_stream_gemm();
+bool stream_gemm_fits(int kblocks, int max_tiles, int num_sms);   // its per-CTA tables hold such a call
 
 cudaError_t launch_wait_timeout_selftest(int* status, cudaStream_t stream);
 
