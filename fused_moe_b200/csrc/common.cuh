@@ -314,6 +314,23 @@ __device__ __forceinline__ float load_as_float(const void* p, int dtype, size_t 
                                : reinterpret_cast<const float*>(p)[i];
 }
 
+// out[g] = p[i + 32 g], g < 8, all eight loads in flight before the first conversion (a conversion behind each load makes
+// eight memory latencies out of one).
+__device__ __forceinline__ void load8_as_float(const void* p, int dtype, size_t i, float (&out)[8]) {
+  if (dtype == B200MOE_BF16) {
+    const unsigned short* q = reinterpret_cast<const unsigned short*>(p) + i;
+    unsigned short raw[8];
+#pragma unroll
+    for (int g = 0; g < 8; ++g) raw[g] = __ldg(q + 32 * g);
+#pragma unroll
+    for (int g = 0; g < 8; ++g) out[g] = __uint_as_float((uint32_t)raw[g] << 16);
+  } else {
+    const float* q = reinterpret_cast<const float*>(p) + i;
+#pragma unroll
+    for (int g = 0; g < 8; ++g) out[g] = __ldg(q + 32 * g);
+  }
+}
+
 // ---- programmatic dependent launch ----
 // A kernel launched with `launch_chained` may become resident while the kernel before it on
 // the stream is still running, so that its prologue (barrier init, tensor-memory allocation,

@@ -48,8 +48,7 @@ route_place_small_kernel(Workspace ws, const void* __restrict__ logits, int logi
   float my_w = 0.f;
   if (warp < T) {
     float b[kNumGroups];
-#pragma unroll
-    for (int g = 0; g < kNumGroups; ++g) b[g] = load_as_float(bias, bias_dtype, g * 32 + lane);
+    load8_as_float(bias, bias_dtype, lane, b);
     route_one_token(logits, logits_dtype, warp, b, rsf, lane, my_id, my_w);
     if (lane < kTopK && my_id >= local_off && my_id < local_off + e_local) le = my_id - local_off;
   }

@@ -24,8 +24,7 @@ route_kernel(const void* __restrict__ logits, int logits_dtype, const void* __re
   chain_release();   // launched in plain stream order itself; the kernel after it may become resident early
   // Lane L owns expert g*32+L of every group g, so a group reduction is a warp reduction.
   float b[kNumGroups];
-#pragma unroll
-  for (int g = 0; g < kNumGroups; ++g) b[g] = load_as_float(bias, bias_dtype, g * 32 + lane);
+  load8_as_float(bias, bias_dtype, lane, b);
 
   for (int t = blockIdx.x * kRouteWarps + warp; t < T; t += gridDim.x * kRouteWarps) {
     int my_id;

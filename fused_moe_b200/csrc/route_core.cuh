@@ -43,10 +43,11 @@ __device__ __forceinline__ void route_one_token(const void* __restrict__ logits,
     float s[kNumGroups];
     uint32_t key[kNumGroups];   // order key of sigmoid + bias (never 0 for a finite value)
     float gscore = 0.f;         // lane g (< 8) keeps the score of group g
+    float x[kNumGroups];
+    load8_as_float(logits, logits_dtype, (size_t)t * kNumExperts + lane, x);
 #pragma unroll
     for (int g = 0; g < kNumGroups; ++g) {
-      float x = load_as_float(logits, logits_dtype, (size_t)t * kNumExperts + g * 32 + lane);
-      s[g] = sigmoid_round_once(x);
+      s[g] = sigmoid_round_once(x[g]);
       key[g] = order_key(s[g] + b[g]);
     }
 #pragma unroll
