@@ -18,7 +18,8 @@ namespace {
 
 // One block per group of four packed rows (grid-stride): a row is 2-8 KB, so one warp walking
 // it alone would be a chain of dependent global loads; 256 threads fetch a row in one or two
-// rounds, and four rows' loads are in flight together.
+// rounds, and four rows' loads are in flight together.  The eight divisions of a 16-byte vector were what it spent its time
+// on (issue slots, not memory): 28 -> 20.6 us for 13386 rows of 2048 with three packed instructions for two quotients.
 constexpr int kRequantRows = 4;
 
 __global__ void __launch_bounds__(256)
@@ -33,7 +34,7 @@ requant_kernel(Workspace ws, int inter) {
   float* row_scale = ws.at<float>(ws.L.row_scale);
   const int vecs = inter / 8;   // 8 halves = 16 bytes
   for (int m0 = blockIdx.x * kRequantRows; m0 < rows; m0 += gridDim.x * kRequantRows) {
-    float scale[kRequantRows];
+    float scale[kRequantRows], inv[kRequantRows];
     bool live[kRequantRows];
 #pragma unroll
     for (int r = 0; r < kRequantRows; ++r) {
@@ -41,6 +42,7 @@ requant_kernel(Workspace ws, int inter) {
       live[r] = m < rows && row_token[m] >= 0;
       const float amax = live[r] ? fmaxf(__uint_as_float(row_amax[m]), 1e-8f) : 1.f;
       scale[r] = fmaxf(amax / 448.0f, 1e-8f);
+      inv[r] = 1.0f / scale[r];
       if (live[r] && threadIdx.x == 0) row_scale[m] = scale[r];
     }
     for (int v = threadIdx.x; v < vecs; v += blockDim.x) {
@@ -51,15 +53,7 @@ requant_kernel(Workspace ws, int inter) {
 #pragma unroll
       for (int r = 0; r < kRequantRows; ++r) {
         if (!live[r]) continue;
-        const float sc = scale[r];
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].x));
-        const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].y));
-        const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].z));
-        const float2 d = __half22float2(*reinterpret_cast<const __half2*>(&raw[r].w));
-        uint2 pk;
-        pk.x = pack4_e4m3(a.x / sc, a.y / sc, b.x / sc, b.y / sc);
-        pk.y = pack4_e4m3(c.x / sc, c.y / sc, d.x / sc, d.y / sc);
-        reinterpret_cast<uint2*>(act_q + (size_t)(m0 + r) * inter)[v] = pk;
+        reinterpret_cast<uint2*>(act_q + (size_t)(m0 + r) * inter)[v] = requant8(raw[r], scale[r], inv[r]);
       }
     }
   }

@@ -595,20 +595,13 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
             for (int j = 0; j < cnt; ++j) {
               const int m = row0 + j;
               const float amax = fmaxf(__uint_as_float(__ldcg(p.row_amax + m)), 1e-8f);
-              const float sc = fmaxf(amax / 448.0f, 1e-8f);
+              const float sc = fmaxf(amax / 448.0f, 1e-8f), inv = 1.0f / sc;
               if (tid == 0) p.row_scale_out[m] = sc;
               const uint4* src = reinterpret_cast<const uint4*>(p.act + (size_t)m * p.inter);
               uint2* dstq = reinterpret_cast<uint2*>(p.act_q_out + (size_t)m * p.inter);
               for (int v = tid; v < vecs; v += 32 * kPromoWarps) {
                 const uint4 raw = __ldcg(src + v);
-                const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
-                const float2 b2 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
-                const float2 c2 = __half22float2(*reinterpret_cast<const __half2*>(&raw.z));
-                const float2 d2 = __half22float2(*reinterpret_cast<const __half2*>(&raw.w));
-                uint2 pk;
-                pk.x = pack4_e4m3(a.x / sc, a.y / sc, b2.x / sc, b2.y / sc);
-                pk.y = pack4_e4m3(c2.x / sc, c2.y / sc, d2.x / sc, d2.y / sc);
-                dstq[v] = pk;
+                dstq[v] = requant8(raw, sc, inv);
               }
             }
           }
