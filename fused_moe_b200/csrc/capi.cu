@@ -141,6 +141,7 @@ int make_tmap_gate_up_kblocks(CUtensorMap* map, const void* base, uint64_t e_loc
 
 uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
+constexpr long long kZeroInGemmBytes = 126ll << 20;   // L2
 constexpr int kDirectRowsMaxTokens = 8;   // largest call whose decode GEMM1 reads the caller's rows in place
 
 // Decode-size calls (up to 16 tokens) requantise inside GEMM1 (B200MOE_DECODE=0 turns that off, B200MOE_DECODE=64
@@ -400,11 +401,15 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   // with inputs cold in HBM: -4 us at 1 token, -2 at 4, but +2..4 at 16 tokens with 4 rows (56 separate 128-byte
   // pieces per row instead of one coalesced pass), hence the limit.
   const bool direct_a = placed && nt == 16 && T <= kDirectRowsMaxTokens && !segs && !segs_dev;
-  // (the gather kernel also zeroes the output rows, which GEMM2's epilogue adds into)
+  // The output rows, which GEMM2's epilogue adds into, are zeroed by the gather pass; by GEMM1 without a gather pass, and by
+  // the grouped GEMM1 when the output is larger than L2 (14107 tokens: a call 873 -> 856 us; below that the zeros stay in L2
+  // until GEMM2 and cost the gather little: 901 tokens 223 -> 228, 8192 rows of an expert-parallel rank 857 -> 864).
+  const bool zero_in_gemm = !slab_nt && (long long)T * hidden * 2 > kZeroInGemmBytes;
   if (!direct_a)
     CUDA_TRY(launch_permute(ws, topk_ids, ids_row_stride, topk_w, w_row_stride, hidden_states, hidden_row_stride,
                             hidden_scale, scale_stride_t, scale_stride_kb, T, e_local, local_expert_offset, hidden,
-                            kTileM, num_sms, st, placed, segs, out_bf16, out_row_stride, segs_dev, n_rows_dev));
+                            kTileM, num_sms, st, placed, segs, out_bf16, out_row_stride, !zero_in_gemm, segs_dev,
+                            n_rows_dev));
 
   GemmParams g1;
   memset(&g1, 0, sizeof(g1));
@@ -439,7 +444,8 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g1.act_q_out = ws.at<uint8_t>(ws.L.act_q);
   g1.row_scale_out = ws.at<float>(ws.L.row_scale);
   g1.direct_a = direct_a ? 1 : 0;
-  g1.zero_tokens = direct_a ? T : 0;   // no gather pass: GEMM1's CTAs zero the output rows that GEMM2 adds into
+  g1.zero_tokens = direct_a || zero_in_gemm ? T : 0;
+  g1.zero_rows_dev = n_rows_dev;
   g1.out = reinterpret_cast<__nv_bfloat16*>(out_bf16);
   g1.out_stride = out_row_stride;
   g1.hscale = hidden_scale;

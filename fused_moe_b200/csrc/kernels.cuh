@@ -39,7 +39,7 @@ cudaError_t launch_permute(const Workspace& ws, const int32_t* ids, long long id
                            long long w_stride, const uint8_t* hidden, long long hidden_row_stride,
                            const float* hscale, long long sstride_t, long long sstride_kb, int T, int e_local,
                            int local_off, int hidden_dim, int pad_rows, int num_sms, cudaStream_t stream,
-                           bool placed, const RowSegments* segs, void* out_bf16, long long out_row_stride,
+                           bool placed, const RowSegments* segs, void* out_bf16, long long out_row_stride, bool zero_out,
                            const RowSegments* segs_dev = nullptr, const int* n_rows_dev = nullptr);
 
 // Routing + scan + placement of at most kFrontSmallMaxTokens tokens in one block (front_small.cu);
@@ -83,7 +83,8 @@ struct GemmParams {
   // decode GEMM1 without a gather pass: tmap_a covers the caller's hidden states [T][K] with one-row boxes, a row's
   // 1x128 scales are read at hscale[token * hs_stride_t + kb * hs_stride_kb]
   int direct_a;
-  int zero_tokens;          // ... and this many rows of `out` are zeroed by GEMM1's CTAs (GEMM2 adds into them)
+  int zero_tokens;          // GEMM1: rows of `out` that its CTAs zero (GEMM2 adds into them); 0 where the gather pass does
+  const int* zero_rows_dev; // optional, device: how many of those rows there are
   const float* hscale;
   long long hs_stride_t, hs_stride_kb;
   int* status;

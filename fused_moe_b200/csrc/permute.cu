@@ -147,8 +147,8 @@ gather_kernel(Workspace ws, const uint8_t* __restrict__ hidden, long long hidden
   if (n_rows_dev) T = min(T, *n_rows_dev);
   // The layer's output starts as zeros: GEMM2's epilogue adds every packed row into its token's row, and a
   // token that no local expert took stays exactly 0.  Zeroed here, by all blocks, instead of by a memset
-  // of its own (one launch boundary less; this kernel runs before the GEMMs in every call).
-  {
+  // of its own (one launch boundary less), unless the grouped GEMM1 does it.
+  if (out) {
     const int vec_per_row = hidden_dim / 8;   // 8 bf16 = 16 bytes
     const long long total = (long long)T * vec_per_row;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -192,7 +192,7 @@ cudaError_t launch_permute(const Workspace& ws, const int32_t* ids, long long id
                            long long w_stride, const uint8_t* hidden, long long hidden_row_stride,
                            const float* hscale, long long sstride_t, long long sstride_kb, int T, int e_local,
                            int local_off, int hidden_dim, int pad_rows, int num_sms, cudaStream_t stream,
-                           bool placed, const RowSegments* segs, void* out_bf16, long long out_row_stride,
+                           bool placed, const RowSegments* segs, void* out_bf16, long long out_row_stride, bool zero_out,
                            const RowSegments* segs_dev, const int* n_rows_dev) {
   const int n_chunks = (T + kChunkTokens - 1) / kChunkTokens;
   cudaError_t err = cudaSuccess;
@@ -217,7 +217,7 @@ cudaError_t launch_permute(const Workspace& ws, const int32_t* ids, long long id
     none.n = 0;
     err = launch_chained(gather_kernel, dim3(blocks), dim3(256), 0, stream, ws, hidden, hidden_row_stride, hscale,
                          sstride_t, sstride_kb, hidden_dim, segs ? *segs : none,
-                         reinterpret_cast<__nv_bfloat16*>(out_bf16), out_row_stride, T, segs_dev, n_rows_dev);
+                         reinterpret_cast<__nv_bfloat16*>(zero_out ? out_bf16 : nullptr), out_row_stride, T, segs_dev, n_rows_dev);
   }
   return err;
 }
