@@ -161,8 +161,9 @@ int decode_tile(int T) {
 // Calls above the decode sizes and up to this many tokens take the weight-streaming GEMMs if few enough experts are local.
 // The 128 x 256 tiles of the grouped kernel come in whole waves of SMs: with some ten to twenty active experts (two waves
 // of GEMM1 items) the second is mostly idle, with more than a hundred it does not matter and the grouped kernel's larger
-// boxes win (56 tokens, 32 experts: 131 -> 115 us with 10 active, 166 -> 163 with 18; 64 tokens, 256 experts: 915 against
-// 945 us).  B200MOE_STREAM=0: never.
+// boxes win (32 experts: 20 tokens 133 -> 117 us with 12 active, 56 tokens 131 -> 115 with 10 and 160 -> 154 with 18, 64
+// tokens on a Zipf load, every expert with some 60 rows, 103 -> 107; 64 tokens over 64 experts 265 -> 250, over 256
+// 915 -> 945).  B200MOE_STREAM=0: never.
 constexpr int kStreamMaxTokens = 64;
 constexpr int kStreamMaxExperts = 64;
 // Returns the most token rows of a tile (an expert of a call of at most 64 tokens has no more), or 0 for the grouped kernels.
@@ -171,7 +172,8 @@ int stream_tile(int T, int e_local) {
     const char* v = getenv("B200MOE_STREAM");
     return !(v && v[0] == '0');
   }();
-  return on && T <= kStreamMaxTokens && e_local <= kStreamMaxExperts ? 64 : 0;
+  // (smaller calls have no scratch for 64 token rows: they stream with decode_tile or not at all)
+  return on && T > 16 && T <= kStreamMaxTokens && e_local <= kStreamMaxExperts ? 64 : 0;
 }
 
 int shape_ok(int T, int e_local, int hidden, int inter) {

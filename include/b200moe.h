@@ -63,7 +63,7 @@ typedef struct b200moe_ws_layout {
   uint64_t total_bytes;
   uint64_t status;        /* int32[16]: [0] status code, [1] detail, [2..] debug */
   uint64_t meta;          /* int32[8]: [0] m_tiles, [1] padded rows, [2] rows with a local expert, [3] pad granularity */
-  uint64_t splitk_count;  /* int32[2][64]: arrivals per (GEMM, weight slab) when a decode GEMM splits K; cleared per call */
+  uint64_t splitk_count;  /* int32[2][160]: arrivals per (GEMM, CTA that begins a cut slab) of the streaming GEMMs; cleared per call */
   uint64_t tile_done;     /* int32[max_tiles]: decode GEMM1, weight slabs of each expert tile already stored; cleared per call */
   uint64_t chunk_counts;  /* int32[n_chunks][e_local] */
   uint64_t chunk_base;    /* int32[n_chunks][e_local] */
@@ -82,7 +82,7 @@ typedef struct b200moe_ws_layout {
   uint64_t topk_ids;      /* int32[T][8]  (used by b200moe_run) */
   uint64_t topk_w;        /* float[T][8]  (used by b200moe_run) */
   uint64_t trace;         /* uint64[2][64][8]: cycle stamps written when B200MOE_PROF is set */
-  uint64_t splitk_scratch; /* float[64][4][16][128]: partial sums of a decode GEMM whose K range is split over CTAs */
+  uint64_t splitk_scratch; /* float[320][nt][128], nt = 16 up to 16 tokens, else 64: partial sums of slabs that the streaming GEMMs cut */
   uint64_t ep_segments;    /* 256 bytes: segment table and row count of b200moe_ep_local_experts (device-written) */
   int32_t m_cap;          /* capacity in packed rows (multiple of 128) */
   int32_t max_tiles;
