@@ -20,6 +20,8 @@ pytestmark = pytest.mark.gpu
     (8, 32, 0, True, 1024, 640),      # rows fetched in place, whole tiles of eight
     (9, 32, 0, True, 1024, 384),      # the first size with a gather pass
     (15, 8, 0, True, 2048, 256),
+    (8, 32, 0, True, 8192, 128),      # the most K blocks, rows in place and gathered
+    (16, 32, 0, True, 8192, 128),
     (16, 32, 0, True, 256, 896),      # a full 16-row tile, K ranges of one group
     (17, 32, 0, True, 512, 128),      # one row past it: 32-row boxes
     (32, 16, 0, True, 256, 384),
