@@ -149,8 +149,10 @@ __device__ __forceinline__ int n_class(int rows) { return rows <= 16 ? 0 : rows 
 
 // Units (K groups) of a CTA's range.  Equal ranges cut tiles anywhere: a CTA then writes up to two sets of partial sums and
 // a tile's last arrival adds several.  Ranges that are whole tiles or an even share of one cost a single set or none, and
-// are taken when they are at most kCutCost units longer (a cut costs about as much).
-constexpr int kCutCost = 4;
+// are taken when they are at most kCutCost units longer (a cut costs about as much).  Measured with 4 / 8 / 12 / 16 / 24 units, us
+// a call: 3 active experts 51.2 / 47.3 / 43.4 / 43.2 / 43.0, 7 active 77.4 / 77.2 / 76.6 / 81.7 / 81.5, 14 active 135.6 / 130.7 /
+// 130.3 / 130.3 / 130.7, 30 active 249 / 241 / 241 / 262 / 261, the others within 1 %.
+constexpr int kCutCost = 12;
 __device__ __forceinline__ int range_of_cta(int units, int groups) {
   const int per = (units + (int)gridDim.x - 1) / (int)gridDim.x;
   if (per == 0) return 0;
