@@ -16,8 +16,8 @@
 //   * the (slab, K group) units of the whole call are cut into one contiguous range per SM, so that every SM reads the same
 //     number of weight bytes; a slab whose range is cut leaves fp32 partial sums in scratch, the CTA that arrives last
 //     adds them in range order and runs the epilogue, so results stay run-to-run identical.
-// Whole calls, 32 experts (11 active, 16 tokens) 157 -> 117 us, 5 active (1 token) 81 -> 61; 256 experts, 4 tokens (30 active,
-// 1.32 GB of weights) 313 -> 247 us, of which GEMM1 167 at 5.3 TB/s and GEMM2 77 at 5.7 TB/s.
+// Whole calls, 32 experts (11 active, 16 tokens) 157 -> 110 us, 5 active (1 token) 81 -> 59; 256 experts, 4 tokens (30 active,
+// 1.32 GB of weights) 313 -> 241 us, of which GEMM1 167 at 5.3 TB/s and GEMM2 77 at 5.7 TB/s.
 // Measured and dropped: GEMM1 and GEMM2 sharing the SMs so that GEMM2's first weights travel early (three and two stages
 // instead of five each: 2 to 4 % slower); three MMA issuers (no change); promotion without its FMAs, boxes without the
 // token rows, another L2 promotion (no change: neither bounds it); tiles of up to 128 token rows for larger calls (901 tokens:
