@@ -330,11 +330,6 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
-__device__ __forceinline__ float load_as_float(const void* p, int dtype, size_t i) {
-  return dtype == B200MOE_BF16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i])
-                               : reinterpret_cast<const float*>(p)[i];
-}
-
 // out[g] = p[i + 32 g], g < 8, all eight loads in flight before the first conversion (a conversion behind each load makes
 // eight memory latencies out of one).
 __device__ __forceinline__ void load8_as_float(const void* p, int dtype, size_t i, float (&out)[8]) {
