@@ -253,7 +253,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
       const int mt = mt0 + threadIdx.x;
       const int e = __ldcg(p.tile_expert + mt);
       const int left = __ldcg(p.expert_count + e) - (mt * kTileM - __ldcg(sp.expert_row0 + e));
-      table[threadIdx.x] = make_int2(e, min(left, NT));   // (more than NT only if a caller's ids repeat within a token)
+      table[threadIdx.x] = make_int2(e, min(left, NT));   // (an expert has no more rows than the call has tokens)
     }
   }
   tc_fence_before();
@@ -624,7 +624,8 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
             }
             transpose8(v, lane);
             const int t = t0 + (lane & 7);
-            if (t < cnt) {
+            const int tok = t < cnt ? p.row_token[row0 + t] : -1;
+            if (tok >= 0) {
               const float rs = p.row_scale[row0 + t] * p.row_weight[row0 + t];
               uint32_t wv[4];
 #pragma unroll
@@ -632,7 +633,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
                 __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * j] * rs, v[2 * j + 1] * rs);
                 wv[j] = *reinterpret_cast<uint32_t*>(&b2);
               }
-              red_add_bf16x8(dst + (size_t)p.row_token[row0 + t] * p.out_stride, wv[0], wv[1], wv[2], wv[3]);
+              red_add_bf16x8(dst + (size_t)tok * p.out_stride, wv[0], wv[1], wv[2], wv[3]);
             }
           }
         }

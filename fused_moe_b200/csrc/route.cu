@@ -39,16 +39,28 @@ route_kernel(const void* __restrict__ logits, int logits_dtype, const void* __re
   }
 }
 
+// A token that names an expert more than once is one row of it, as the placement makes it (permute.cu): every pair but the
+// last is left out here too.  Counted, they would leave rows between the placed ones and the expert's padding whose token
+// nobody writes, and the GEMMs' epilogues store by that token.  (The ids that the routing kernels count themselves differ.)
 __global__ void __launch_bounds__(256)
 count_kernel(const int32_t* __restrict__ ids, long long row_stride, int T, int local_off, int e_local,
              int* __restrict__ chunk_counts, const int* __restrict__ n_rows_dev) {
   chain_release();
   if (n_rows_dev) T = min(T, *n_rows_dev);
-  long long n = (long long)T * kTopK;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    int t = (int)(i / kTopK), k = (int)(i % kTopK);
-    int le = ids[(size_t)t * row_stride + k] - local_off;
-    if (le >= 0 && le < e_local) atomicAdd(&chunk_counts[(t / kChunkTokens) * e_local + le], 1);
+  const long long n = (long long)T * kTopK;
+  const int lane = threadIdx.x & 31;
+  // a token's pairs lie in eight neighbouring lanes; whole warps stay in the loop for the shuffles
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i - lane < n; i += (long long)gridDim.x * blockDim.x) {
+    const int t = (int)(i / kTopK), k = (int)(i % kTopK);
+    const int id = i < n ? ids[(size_t)t * row_stride + k] : -1;
+    bool last = true;
+#pragma unroll
+    for (int d = 1; d < kTopK; ++d) {
+      const int other = __shfl_down_sync(0xffffffffu, id, d, kTopK);
+      if (k + d < kTopK && other == id) last = false;
+    }
+    const int le = id - local_off;
+    if (i < n && last && le >= 0 && le < e_local) atomicAdd(&chunk_counts[(t / kChunkTokens) * e_local + le], 1);
   }
 }
 

@@ -140,7 +140,8 @@ B200MOE_API const char* b200moe_route_static_error(void);
 
 /* Histogram of local experts for routing that was computed elsewhere (the
  * expert-parallel path, where rows arrive with their ids).  Clears and fills the same
- * workspace counters as b200moe_route.  ids_row_stride in int32 elements. */
+ * workspace counters as b200moe_route.  ids_row_stride in int32 elements.  The eight ids of a
+ * token should differ: an expert named more than once is one row, with the last one's weight. */
 B200MOE_API int b200moe_count(const int32_t* topk_ids, int64_t ids_row_stride, int T,
                   int local_expert_offset, int e_local, int hidden, int inter,
                   void* workspace, size_t workspace_bytes, void* stream);
