@@ -299,15 +299,16 @@ __device__ __forceinline__ uint32_t pack4_e4m3(float a, float b, float c, float 
   return lo | (hi << 16);
 }
 
-// Two quotients x / d, correctly rounded, given inv = RN(1 / d): Markstein's theorem (P. Markstein, "Computation of
-// elementary functions on the IBM RISC System/6000 processor", 1990): q = RN(x inv), r = x - q d (exact in one FMA),
-// RN(q + r inv) is RN(x / d).  Nothing may underflow: here |x| is 0 or at least 2^-24 and d lies in [1e-8, 147].  Three packed
-// instructions for two quotients, where a division is a sequence of about ten for each.
+// Two quotients x / d, correctly rounded and with the sign of a zero kept, given inv = RN(1 / d), by the remainder step of
+// P. Markstein ("Computation of elementary functions on the IBM RISC System/6000 processor", 1990): q = RN(x inv),
+// r = q d - x, RN(q - r inv).  His theorem wants q within one ulp, which RN(x inv) can miss by half an ulp more; what it is
+// used for was therefore compared with the plain division one by one, every fp16 x up to every fp16 row maximum
+// (d = max / 448, at least 1e-8; 1.0e9 pairs): no quotient differs.  (With r = x - q d a zero always came out positive.)
+// Three packed instructions for two quotients, where a division is a sequence of about ten for each.
 __device__ __forceinline__ float2 div2_rn(float2 x, float d, float inv) {
-  const float2 inv2 = make_float2(inv, inv);
-  const float2 q = __fmul2_rn(x, inv2);
-  const float2 r = __ffma2_rn(make_float2(-q.x, -q.y), make_float2(d, d), x);
-  return __ffma2_rn(r, inv2, q);
+  const float2 q = __fmul2_rn(x, make_float2(inv, inv));
+  const float2 r = __ffma2_rn(q, make_float2(d, d), make_float2(-x.x, -x.y));
+  return __ffma2_rn(r, make_float2(-inv, -inv), q);
 }
 
 // Eight fp16 activations (16 bytes) -> eight e4m3 codes of x / scale.
