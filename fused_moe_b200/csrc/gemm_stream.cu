@@ -31,6 +31,7 @@
 
 #include "common.cuh"
 #include "kernels.cuh"
+#include "stream_plan.cuh"
 
 namespace b200moe {
 
@@ -147,19 +148,6 @@ __device__ __forceinline__ void transpose8(float (&v)[8], int lane) {
 // The token box and the MMA's N for a tile of `rows` real rows: 16, 32 or 64 (log2 - 4 picks the tensor map).
 __device__ __forceinline__ int n_class(int rows) { return rows <= 16 ? 0 : rows <= 32 ? 1 : 2; }
 
-// Units (K groups) of a CTA's range.  Equal ranges cut tiles anywhere: a CTA then writes up to two sets of partial sums and
-// a tile's last arrival adds several.  Ranges that are whole tiles or an even share of one cost a single set or none, and
-// are taken when they are at most kCutCost units longer (a cut costs about as much).  Measured with 4 / 8 / 12 / 16 / 24 units, us
-// a call: 3 active experts 51.2 / 47.3 / 43.4 / 43.2 / 43.0, 7 active 77.4 / 77.2 / 76.6 / 81.7 / 81.5, 14 active 135.6 / 130.7 /
-// 130.3 / 130.3 / 130.7, 30 active 249 / 241 / 241 / 262 / 261, the others within 1 %.
-constexpr int kCutCost = 12;
-__device__ __forceinline__ int range_of_cta(int units, int groups) {
-  const int per = (units + (int)gridDim.x - 1) / (int)gridDim.x;
-  if (per == 0) return 0;
-  const int share = per < groups ? (groups + groups / per - 1) / (groups / per) : (per + groups - 1) / groups * groups;
-  return share - per <= kCutCost ? share : per;
-}
-
 template <int MODE, int NT>
 __global__ void __launch_bounds__(SCfg<MODE, NT>::kThreads, 1)
 stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
@@ -240,7 +228,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
   const int KB = p.kblocks, K = (KB + G - 1) / G;   // K blocks, and the groups that are the units of work
   const int box_kb = min(G, KB);                    // K blocks of a box (past the end of K they are filled with zeros)
   const int units = __ldcg(p.meta) * p.n_tiles * K;
-  const int per_cta = range_of_cta(units, K);       // units of a CTA (the last ones may get none)
+  const int per_cta = stream_range(units, K, (int)gridDim.x);   // units of a CTA (the last ones may get none)
   const int u0 = min(units, (int)blockIdx.x * per_cta);
   const int u1 = min(units, u0 + per_cta);
   const int mt0 = u0 / (K * p.n_tiles);
