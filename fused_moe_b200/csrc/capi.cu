@@ -142,6 +142,7 @@ int make_tmap_gate_up_kblocks(CUtensorMap* map, const void* base, uint64_t e_loc
 uint64_t align_up(uint64_t x, uint64_t a) { return (x + a - 1) / a * a; }
 
 constexpr long long kZeroInGemmBytes = 126ll << 20;   // L2
+constexpr int kZeroInGemmExperts = 4;
 constexpr int kDirectRowsMaxTokens = 8;   // largest call whose decode GEMM1 reads the caller's rows in place
 
 // Decode-size calls (up to 16 tokens) requantise inside GEMM1 (B200MOE_DECODE=0 turns that off, B200MOE_DECODE=64
@@ -404,9 +405,15 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   // pieces per row instead of one coalesced pass), hence the limit.
   const bool direct_a = placed && nt == 16 && T <= kDirectRowsMaxTokens && !segs && !segs_dev;
   // The output rows, which GEMM2's epilogue adds into, are zeroed by the gather pass; by GEMM1 without a gather pass, and by
-  // the grouped GEMM1 when the output is larger than L2 (14107 tokens: a call 873 -> 856 us; below that the zeros stay in L2
-  // until GEMM2 and cost the gather little: 901 tokens 223 -> 228, 8192 rows of an expert-parallel rank 857 -> 864).
-  const bool zero_in_gemm = !slab_nt && (long long)T * hidden * 2 > kZeroInGemmBytes;
+  // the grouped GEMM1 when the output is larger than L2 and in one piece, and more than three experts are local.  Below the size
+  // of L2 the zeros stay there until GEMM2 and cost the gather little (901 tokens: gather 223, GEMM1 228 us a call; 8192 rows of
+  // an expert-parallel rank 857, 864).  With few local experts GEMM1 is too short to hide 148 CTAs' stores behind its K
+  // loops, and a padded row stride takes a division per 16 bytes.  us a call zeroed by the gather pass / GEMM1, output in one piece:
+  // 1 expert, 14107 tokens 124.9 / 137.2, 30001 tokens 192.5 / 210.9; 2: 139.3 / 141.3, 204.8 / 213.0; 3: 143.4 / 149.5,
+  // 213.0 / 215.2; 4: 249.9 / 245.8, 440.3 / 423.9; 8: 311.3 / 309.3, 591.9 / 583.7; 32: 964.6 / 948.1; 64: 1716 / 1700.
+  // Padded rows, 14107 tokens: 1 expert 124.9 / 155.6; 4: 251.9 / 264.2; 32: 950.3 / 956.5; 64: 1718 / 1739.
+  const bool zero_in_gemm = !slab_nt && (long long)T * hidden * 2 > kZeroInGemmBytes && e_local >= kZeroInGemmExperts &&
+                            out_row_stride == hidden;
   if (!direct_a)
     CUDA_TRY(launch_permute(ws, topk_ids, ids_row_stride, topk_w, w_row_stride, hidden_states, hidden_row_stride,
                             hidden_scale, scale_stride_t, scale_stride_kb, T, e_local, local_expert_offset, hidden,

@@ -167,29 +167,21 @@ __device__ __forceinline__ bool counter_wait(uint32_t addr, uint32_t target, vol
   }
 }
 
-// GEMM1 of a call whose output is larger than L2 also zeroes the output rows, which GEMM2 adds into: its time goes into the
-// hand-off chain of the tensor cores and leaves HBM idle, while the gather pass, which does it otherwise, is bound by HBM.  CTA b of G clears the b-th
-// of G equal shares, the i-th of its n items the i-th part of that: `step` of `steps` (parts of 256 threads x 16 bytes).
-// (32-expert slice at 14107 tokens, 202 MB of output: gather 76 -> 35 us, the call 873 -> 856.)
+// GEMM1 of a call whose output is larger than L2 also zeroes the output rows (one piece of memory), which GEMM2 adds into: its
+// time goes into the hand-off chain of the tensor cores and leaves HBM idle, while the gather pass, which does it otherwise, is
+// bound by HBM.  CTA b of G clears the b-th of G equal shares, the i-th of its n items the i-th part of that: `step` of `steps`
+// (parts of 256 threads x 16 bytes).  (32-expert slice at 14107 tokens, 202 MB of output: gather 76 -> 35 us, the call 873 -> 856.)
 __device__ __forceinline__ void zero_output(const GemmParams& p, int tid, int step, int steps) {
   const int rows = p.zero_rows_dev ? min(p.zero_tokens, *p.zero_rows_dev) : p.zero_tokens;
-  const uint32_t vec_per_row = p.hidden / 8;   // 8 bf16 = 16 bytes
-  const long long total = (long long)rows * vec_per_row;
+  const long long total = (long long)rows * (p.hidden / 8);   // 8 bf16 = 16 bytes
   const long long share = (total + gridDim.x - 1) / gridDim.x;
   const long long part = (share + steps - 1) / steps;
   const long long begin = blockIdx.x * share + step * part;
   long long end = begin + part;
   if (end > (blockIdx.x + 1) * share) end = (blockIdx.x + 1) * share;
   if (end > total) end = total;
-  const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-  if (p.out_stride == p.hidden) {
-    for (long long i = begin + tid; i < end; i += 32 * kPromoWarps) reinterpret_cast<uint4*>(p.out)[i] = zero;
-  } else {
-    for (long long i = begin + tid; i < end; i += 32 * kPromoWarps) {
-      const long long t = i / vec_per_row;
-      reinterpret_cast<uint4*>(p.out + t * p.out_stride)[i - t * vec_per_row] = zero;
-    }
-  }
+  for (long long i = begin + tid; i < end; i += 32 * kPromoWarps)
+    reinterpret_cast<uint4*>(p.out)[i] = make_uint4(0u, 0u, 0u, 0u);
 }
 
 template <int MODE, bool PROF>
