@@ -221,10 +221,17 @@ void compute_layout(int T, int e_local, int hidden, int inter, b200moe_ws_layout
   L->topk_ids = take((uint64_t)(T > 0 ? T : 1) * kTopK * 4);
   L->topk_w = take((uint64_t)(T > 0 ? T : 1) * kTopK * 4);
   L->trace = take(2 * 8 * 64 * 8);   // B200MOE_PROF: absolute cycle stamps of CTA 0's first 64 K blocks
-  // two cut tiles per CTA of the streaming GEMMs: 2.5 MiB at decode sizes, 10 MiB (64 token rows) above
-  L->splitk_scratch = take((uint64_t)2 * kStreamMaxCtas * (T <= 16 ? 16 : 64) * 128 * 4);
+  // two cut tiles per CTA of the streaming GEMMs: 2.5 MiB at decode sizes, 10 MiB (64 token rows) up to kStreamMaxTokens, above
+  // which no call streams
+  const int stream_rows = T <= 16 ? 16 : T <= kStreamMaxTokens ? 64 : 0;
+  L->splitk_scratch = take((uint64_t)2 * kStreamMaxCtas * stream_rows * 128 * 4);
   L->ep_segments = take(256);   // RowSegments at +0, int32 row count at +192 (b200moe_ep_local_experts)
   L->total_bytes = off;
+  if (T > kStreamMaxTokens) {   // a workspace for so many tokens holds every smaller call, the largest that streams among them
+    b200moe_ws_layout at_limit;
+    compute_layout(kStreamMaxTokens, e_local, hidden, inter, &at_limit);
+    if (at_limit.total_bytes > off) L->total_bytes = at_limit.total_bytes;
+  }
 }
 
 int bind_workspace(int T, int e_local, int hidden, int inter, void* workspace, size_t bytes, Workspace* ws) {

@@ -53,6 +53,17 @@ def test_workspace_layout_is_aligned_ordered_and_grows_with_T():
     assert _capi.workspace_layout(4096, 256, 7168, 2048).total_bytes < 4 * 2 ** 30
 
 
+@pytest.mark.parametrize("e,h,i", [(1, 256, 128), (8, 512, 256), (32, 7168, 2048), (256, 7168, 2048)])
+def test_workspace_holds_every_smaller_call_and_no_streaming_scratch_above_64_tokens(e, h, i):
+    totals = []
+    for T in range(1, 400):
+        L = _capi.workspace_layout(T, e, h, i)
+        scratch = L.ep_segments - L.splitk_scratch
+        assert scratch == 320 * (16 if T <= 16 else 64 if T <= 64 else 0) * 128 * 4, T
+        totals.append(L.total_bytes)
+    assert totals == sorted(totals)
+
+
 @pytest.mark.parametrize("T,e,h,i,code", [
     (-1, 32, 7168, 2048, -1), (8, 0, 7168, 2048, -1), (8, 257, 7168, 2048, -2),
     (8, 32, 7000, 2048, -2), (8, 32, 7168, 2000, -2), (8, 32, 128, 2048, -2),
