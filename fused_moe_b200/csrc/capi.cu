@@ -249,11 +249,14 @@ int bind_workspace(int T, int e_local, int hidden, int inter, void* workspace, s
 uint32_t group_kblocks(int k) { return k / kBlockK < kStreamGroup ? k / kBlockK : kStreamGroup; }
 
 // What the streaming kernels take beside a GEMM's ordinary arguments: the packed rows ([m_cap][k] at `rows_off`) in boxes
-// of 16, 32 and 64 rows.
-int make_stream_params(StreamParams* sp, const GemmParams& g, const Workspace& ws, uint64_t rows_off, int k) {
+// of 16 rows and, where a tile may hold more (`nt` 64), 32 and 64.  Only what the kernel reads is encoded: a map costs the host a
+// good part of a microsecond, and a call at new addresses pays for each.
+int make_stream_params(StreamParams* sp, const GemmParams& g, const Workspace& ws, uint64_t rows_off, int k, int nt) {
+  memset(sp, 0, sizeof(*sp));
   sp->g = g;
   sp->expert_row0 = ws.at<int>(ws.L.expert_row0);
-  for (int c = 0; c < 3; ++c) {
+  const int n_maps = g.direct_a ? 0 : nt <= 16 ? 1 : 3;
+  for (int c = 0; c < n_maps; ++c) {
     const int rc = make_tmap_kblocks(&sp->tmap_tok[c], ws.base + rows_off, (uint64_t)ws.L.m_cap, (uint64_t)k, 16u << c,
                                      group_kblocks(k));
     if (rc != B200MOE_OK) return rc;
@@ -433,8 +436,8 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
     if ((rc = make_tmap(&g1.tmap_a, hidden_states, (uint64_t)T, (uint64_t)hidden, (uint64_t)hidden_row_stride, 1)) !=
         B200MOE_OK)
       return rc;
-  } else if ((rc = make_tmap(&g1.tmap_a, ws.base + ws.L.a_packed, (uint64_t)ws.L.m_cap, (uint64_t)hidden,
-                             (uint64_t)hidden, kTileM)) != B200MOE_OK) {
+  } else if (!slab_nt && (rc = make_tmap(&g1.tmap_a, ws.base + ws.L.a_packed, (uint64_t)ws.L.m_cap, (uint64_t)hidden,
+                                         (uint64_t)hidden, kTileM)) != B200MOE_OK) {
     return rc;
   }
   // one box = 128 gate rows + the matching 128 up rows (streaming kernels: 64 + 64, a group of K blocks)
@@ -481,7 +484,7 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
     cudaError_t le;
     if (slab_nt) {
       StreamParams s1;
-      if ((rc = make_stream_params(&s1, g1, ws, ws.L.a_packed, hidden)) != B200MOE_OK) return rc;
+      if ((rc = make_stream_params(&s1, g1, ws, ws.L.a_packed, hidden, slab_nt)) != B200MOE_OK) return rc;
       le = launch_stream_gemm(1, slab_nt, s1, ws.L.max_tiles, num_sms, st);
     } else {
       le = launch_grouped_gemm(1, g1, num_sms, st);
@@ -498,7 +501,8 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
 
   GemmParams g2;
   memset(&g2, 0, sizeof(g2));
-  if ((rc = make_tmap(&g2.tmap_a, ws.base + ws.L.act_q, (uint64_t)ws.L.m_cap, (uint64_t)inter, (uint64_t)inter,
+  if (!slab_nt &&
+      (rc = make_tmap(&g2.tmap_a, ws.base + ws.L.act_q, (uint64_t)ws.L.m_cap, (uint64_t)inter, (uint64_t)inter,
                       kTileM)) != B200MOE_OK)
     return rc;
   // the whole B tile (or the 128-row slab of a group of K blocks) in one box
@@ -528,7 +532,7 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g2.trace = prof_on ? ws.at<unsigned long long>(ws.L.trace) + 8 * 64 : nullptr;
   if (slab_nt) {
     StreamParams s2;
-    if ((rc = make_stream_params(&s2, g2, ws, ws.L.act_q, inter)) != B200MOE_OK) return rc;
+    if ((rc = make_stream_params(&s2, g2, ws, ws.L.act_q, inter, slab_nt)) != B200MOE_OK) return rc;
     CUDA_TRY(launch_stream_gemm(2, slab_nt, s2, ws.L.max_tiles, num_sms, st));
   } else {
     CUDA_TRY(launch_grouped_gemm(2, g2, num_sms, st));

@@ -55,7 +55,7 @@ constexpr int kStreamMaxCtas = 160;
 constexpr int kStreamGroup = 2;   // K blocks that travel and are handed over together
 
 // Arguments of the two grouped GEMMs.  `tmap_a` covers the packed rows [m_cap][K],
-// `tmap_b` the weights viewed as [e_local * N][K]; both e4m3, 128-byte swizzled boxes.
+// `tmap_b` the weights viewed as [e_local * N][K]; both e4m3, 128-byte swizzled boxes (`tmap_a`: see StreamParams).
 struct GemmParams {
   CUtensorMap tmap_a;
   CUtensorMap tmap_b;
@@ -105,7 +105,7 @@ int grouped_gemm_max_kblocks();         // largest K / 128 the kernels' scale pa
 struct StreamParams {
   GemmParams g;               // tmap_b: boxes of kStreamGroup K blocks x 64 gate + 64 up rows (GEMM1), 128 rows (GEMM2); tmap_a:
                               // direct_a only (one row, one K block)
-  CUtensorMap tmap_tok[3];    // the packed rows in boxes of kStreamGroup K blocks x 16, 32, 64 rows
+  CUtensorMap tmap_tok[3];    // the packed rows in boxes of kStreamGroup K blocks x 16, 32, 64 rows (nt 16: the first; direct_a: none)
   const int* expert_row0;
 };
 cudaError_t launch_stream_gemm(int mode, int nt, const StreamParams& p, int max_tiles, int num_sms, cudaStream_t stream);
