@@ -565,18 +565,15 @@ def run_profile_case(args):
     meta = ws.view("meta", torch.int32, (8,)).cpu().numpy()
     counts = ws.view("expert_count", torch.int32, (E,)).cpu().numpy()
     prof = None
-    if os.environ.get("B200MOE_PROF") and args.tokens > 64:   # (the streaming kernels of smaller calls keep no counters)
+    if os.environ.get("B200MOE_PROF"):
         raw = ws.view("meta", torch.int64, (32,)).cpu().numpy()      # meta + its padding, as u64 words
         names = ("wait_acc", "promote", "mma_issue", "kblocks", "epi_role_total", "tile_epilogues", "unused2",
                  "mma_wait_epilogue", "mma_wait_tma")
+        if raw[13]:    # the streaming kernels' counters
+            names = ("prod_wait_stage", "prod_issue", "prod_total", "kgroups", "mma_wait_acc", "mma_wait_tma",
+                     "mma_issue", "promo_wait_acc", "promo_total")
         prof = {"gemm1": dict(zip(names, (int(x) for x in raw[4:13]))),
                 "gemm2": dict(zip(names, (int(x) for x in raw[17:26])))}
-        # eight cycle stamps per K block of CTA 0: issuer wait start, operands landed, accumulator free,
-        # MMAs issued; promotion warp 0: accumulator ready, first chunks read, accumulator released, done
-        tr = ws.view("trace", torch.int64, (2, 64, 8)).cpu().numpy()
-        for name, t in (("gemm1", tr[0]), ("gemm2", tr[1])):
-            base = int(t[8, 0])
-            prof[name]["trace_kb8_31"] = [[int(x) - base for x in t[i]] for i in range(8, 32)]
     print(json.dumps({"profile_case": f"slice{E}", "tokens": args.tokens, "zipf": args.zipf, "status": code,
                       "cycle_counters_cta0": prof,
                       "ms_per_call": a.elapsed_time(b) / max(args.steps, 1), "rows": int(meta[2]),

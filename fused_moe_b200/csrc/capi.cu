@@ -220,7 +220,7 @@ void compute_layout(int T, int e_local, int hidden, int inter, b200moe_ws_layout
   L->tok_rows = take((uint64_t)(T > 0 ? T : 1) * kTopK * 4);
   L->topk_ids = take((uint64_t)(T > 0 ? T : 1) * kTopK * 4);
   L->topk_w = take((uint64_t)(T > 0 ? T : 1) * kTopK * 4);
-  L->trace = take(2 * 8 * 64 * 8);   // B200MOE_PROF: absolute cycle stamps of CTA 0's first 64 K blocks
+  L->trace = take(2 * 8 * 64 * 8);   // room for one-off probes: absolute cycle stamps of CTA 0's first 64 K blocks
   // two cut tiles per CTA of the streaming GEMMs: 2.5 MiB at decode sizes, 10 MiB (64 token rows) up to kStreamMaxTokens, above
   // which no call streams
   const int stream_rows = T <= 16 ? 16 : T <= kStreamMaxTokens ? 64 : 0;
@@ -474,11 +474,10 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g1.status_mirror = g_status_mirror;
   g1.splitk_scratch = ws.at<float>(ws.L.splitk_scratch);
   g1.splitk_count = ws.at<int>(ws.L.splitk_count);
-  // B200MOE_PROF=1: CTA 0 adds cycle counters into the padding after `meta`
-  // (GEMM1: 9 x u64 at meta+32, GEMM2: at meta+136); cleared with the counters each call.
+  // B200MOE_PROF=1: CTA 0 writes its cycle counters into the padding after `meta` (GEMM1: 10 x u64 at meta+32, GEMM2: at
+  // meta+136; the last word tells the streaming kernels' from the grouped ones'); cleared with the counters each call.
   static const bool prof_on = getenv("B200MOE_PROF") != nullptr;
   g1.prof = prof_on ? ws.at<unsigned long long>(ws.L.meta + 32) : nullptr;
-  g1.trace = prof_on ? ws.at<unsigned long long>(ws.L.trace) : nullptr;
   if (g_prof_start) CUDA_TRY(cudaEventRecord(g_prof_start, st));
   {
     cudaError_t le;
@@ -529,7 +528,6 @@ static int experts_impl(const int32_t* topk_ids, int64_t ids_row_stride, const f
   g2.splitk_scratch = g1.splitk_scratch;
   g2.splitk_count = g1.splitk_count + kStreamMaxCtas;
   g2.prof = prof_on ? ws.at<unsigned long long>(ws.L.meta + 136) : nullptr;
-  g2.trace = prof_on ? ws.at<unsigned long long>(ws.L.trace) + 8 * 64 : nullptr;
   if (slab_nt) {
     StreamParams s2;
     if ((rc = make_stream_params(&s2, g2, ws, ws.L.act_q, inter, slab_nt)) != B200MOE_OK) return rc;

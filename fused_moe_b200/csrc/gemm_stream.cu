@@ -148,7 +148,8 @@ __device__ __forceinline__ void transpose8(float (&v)[8], int lane) {
 // The token box and the MMA's N for a tile of `rows` real rows: 16, 32 or 64 (log2 - 4 picks the tensor map).
 __device__ __forceinline__ int n_class(int rows) { return rows <= 16 ? 0 : rows <= 32 ? 1 : 2; }
 
-template <int MODE, int NT>
+// PROF (B200MOE_PROF=1): CTA 0's cycle counters, g.prof[0 .. 8], and a 1 in g.prof[9] (the grouped kernels' differ).
+template <int MODE, int NT, bool PROF>
 __global__ void __launch_bounds__(SCfg<MODE, NT>::kThreads, 1)
 stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
   using Cfg = SCfg<MODE, NT>;
@@ -297,6 +298,8 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
       // was through with the scales of group it - S - 5.
       uint32_t it = 0;
       bool alive = true;
+      long long t_wait = 0, t_issue = 0;
+      const long long t_begin = PROF ? clock64() : 0;
       for (int u = u0; u < u1 && alive;) {
         const int tile = u / K, kb0 = u - tile * K;
         const int len = min(K - kb0, u1 - u);
@@ -306,8 +309,11 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
         for (int kb = kb0; kb < kb0 + len; ++kb, ++it) {
           if ((it % kProducers) != pme) continue;
           const uint32_t s = it % S, ph = (it / S) & 1u, full = bar_full + 8 * s;
+          const long long q0 = PROF ? clock64() : 0;
+          long long q1 = q0;
           if (it >= early) {
             if (!mbar_wait(bar_empty + 8 * s, ph ^ 1u, abort_flag, p.status, 41)) { alive = false; break; }
+            if (PROF) q1 = clock64();
             mbar_arrive_expect_tx(full, direct ? (uint32_t)(box_kb * kWBytes + min(G, KB - kb * G) * info.y * kBlockK)
                                                : stage_bytes(n, kb));
             load_weights(s, kb, slab, info.x);
@@ -319,16 +325,26 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
               for (int j = 0; j < info.y; ++j)
                 tma_load_2d(tok_dst + (x - kb * G) * Cfg::kTokBytes + j * kBlockK, &p.tmap_a, x * kBlockK,
                             toks[(m_tile - mt0) * 16 + j], full);
-            continue;
+          } else {
+            // n rows of each of the group's K blocks, the K blocks n x 128 bytes apart
+            tma_load_3d(tok_dst, &sp.tmap_tok[cls], 0, m_tile * kTileM, kb * G, full);
+            if (MODE == 1)
+              for (int x = kb * G; x < kb_end; ++x)
+                bulk_load(smem_u32(ring) + ((it % kScaleSlots) * G + (x - kb * G)) * (NT * 4),
+                          p.a_scale + (size_t)x * p.m_cap + (size_t)m_tile * kTileM, n * 4, full);
           }
-          // n rows of each of the group's K blocks, the K blocks n x 128 bytes apart
-          tma_load_3d(tok_dst, &sp.tmap_tok[cls], 0, m_tile * kTileM, kb * G, full);
-          if (MODE == 1)
-            for (int x = kb * G; x < kb_end; ++x)
-              bulk_load(smem_u32(ring) + ((it % kScaleSlots) * G + (x - kb * G)) * (NT * 4),
-                        p.a_scale + (size_t)x * p.m_cap + (size_t)m_tile * kTileM, n * 4, full);
+          if (PROF) {
+            t_wait += q1 - q0;
+            t_issue += clock64() - q1;
+          }
         }
         u += len;
+      }
+      if (PROF && p.prof && blockIdx.x == 0 && pme == 0) {
+        p.prof[0] = (unsigned long long)t_wait;                    // producer 0 waiting for a free stage
+        p.prof[1] = (unsigned long long)t_issue;                   // producer 0 issuing copies
+        p.prof[2] = (unsigned long long)(clock64() - t_begin);     // producer 0: whole loop
+        p.prof[3] = (unsigned long long)it;                        // K groups of the CTA
       }
       // copies still in flight must land before the CTA's shared memory is released
       const uint32_t first = it > (uint32_t)S ? it - S : 0u;
@@ -341,6 +357,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
       const uint32_t me = (uint32_t)(warp - 1);
       uint32_t it = 0;
       bool alive = true;
+      long long t_acc = 0, t_tma = 0, t_issue = 0;
       for (int u = u0; u < u1 && alive;) {
         const int tile = u / K, kb0 = u - tile * K;
         const int len = min(K - kb0, u1 - u);
@@ -351,8 +368,11 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
           if ((it % kIssuers) != me) continue;
           const uint32_t s = it % S, ph = (it / S) & 1u;
           const uint32_t b = it % kAccs, bph = (it / kAccs) & 1u;
+          const long long q0 = PROF ? clock64() : 0;
           if (!mbar_wait(bar_tempty + 8 * b, bph ^ 1u, abort_flag, p.status, 42)) { alive = false; break; }
+          const long long q1 = PROF ? clock64() : 0;
           if (!mbar_wait(bar_full + 8 * s, ph, abort_flag, p.status, 43)) { alive = false; break; }
+          const long long q2 = PROF ? clock64() : 0;
           tc_fence_after();
           const uint32_t w_addr = smem_base + s * Cfg::kStageBytes;
           for (int g = 0; g < G && (kb0 + kb) * G + g < KB; ++g)
@@ -360,11 +380,21 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
                              kmajor_sw128_desc_lo(w_addr + G * kWBytes + g * tok_step), kKmajorSw128DescHi, idesc);
           tc_commit(bar_empty + 8 * s);
           tc_commit(bar_tfull + 8 * b);
+          if (PROF) {
+            t_acc += q1 - q0;
+            t_tma += q2 - q1;
+            t_issue += clock64() - q2;
+          }
         }
         u += len;
       }
       tc_commit(bar_drain + 8 * me);
       (void)mbar_wait(bar_drain + 8 * me, 0u, abort_flag + 1, p.status, 45);
+      if (PROF && p.prof && blockIdx.x == 0 && me == 0) {
+        p.prof[4] = (unsigned long long)t_acc;     // issuer 0 waiting for a free accumulator
+        p.prof[5] = (unsigned long long)t_tma;     // issuer 0 waiting for operands
+        p.prof[6] = (unsigned long long)t_issue;   // issuer 0 issuing MMAs and commits
+      }
     }
   } else {
     // ------------------------------ promotion + epilogue ------------------------------
@@ -373,6 +403,8 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
     float* panel = panels + (warp - 4) * (Cfg::kPanelBytes / 4);   // (rows in place)
     uint32_t it = 0, xi = 0, si = 0, ri = 0;
     bool alive = true;
+    long long t_wait = 0;
+    const long long t_begin = PROF ? clock64() : 0;
     const int nblk_per_expert = p.n_per_expert / kBlockK;
     // weight scales of a tile, two per lane (K block lane and lane + 32)
     auto load_sb = [&](int tile, float& lo, float& hi) {
@@ -411,10 +443,12 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
         const bool two = kb + 1 < KB;               // the last group of an odd K has one K block
         const float sb_half = kb < 32 ? sb_lo : sb_hi;
         const float sb0 = __shfl_sync(0xffffffffu, sb_half, kb & 31), sb1 = __shfl_sync(0xffffffffu, sb_half, (kb + 1) & 31);
+        const long long q0 = PROF ? clock64() : 0;
         bool ok = mbar_wait(bar_tfull + 8 * b, bph, abort_flag, p.status, 44);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) { alive = false; break; }
         tc_fence_after();
+        if (PROF) t_wait += clock64() - q0;
         const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + b * (G * NT) + h * 16;
         const float4* sa = reinterpret_cast<const float4*>(ring + (it % kScaleSlots) * (G * NT) + h * 16);   // GEMM1
         if constexpr (NT == 16) {
@@ -627,6 +661,11 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
         }
       }
     }
+    if (PROF && p.prof && blockIdx.x == 0 && warp == 4 && lane == 0) {
+      p.prof[7] = (unsigned long long)t_wait;                  // promotion warp 0 waiting for an accumulator
+      p.prof[8] = (unsigned long long)(clock64() - t_begin);   // promotion warp 0: whole role
+      p.prof[9] = 1;
+    }
   }
 
   tc_fence_before();
@@ -642,13 +681,17 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
 
 template <int MODE, int NT>
 cudaError_t launch_one(const StreamParams& p, int grid, cudaStream_t stream) {
-  return launch_chained(stream_gemm_kernel<MODE, NT>, dim3(grid), dim3(SCfg<MODE, NT>::kThreads),
-                        SCfg<MODE, NT>::kSmemBytes, stream, p);
+  using Cfg = SCfg<MODE, NT>;
+  return launch_chained(p.g.prof ? stream_gemm_kernel<MODE, NT, true> : stream_gemm_kernel<MODE, NT, false>, dim3(grid),
+                        dim3(Cfg::kThreads), Cfg::kSmemBytes, stream, p);
 }
 
 template <int MODE, int NT>
 cudaError_t configure_one() {
-  return cudaFuncSetAttribute(stream_gemm_kernel<MODE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const cudaError_t e = cudaFuncSetAttribute(stream_gemm_kernel<MODE, NT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             SCfg<MODE, NT>::kSmemBytes);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(stream_gemm_kernel<MODE, NT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               SCfg<MODE, NT>::kSmemBytes);
 }
 

@@ -92,7 +92,6 @@ struct GemmParams {
   float* splitk_scratch;    // streaming GEMMs: [2 per CTA][nt][128] partial sums of cut tiles
   int* splitk_count;        // streaming GEMMs: arrivals at the tile that a CTA begins and others finish, zero at kernel start and end
   unsigned long long* prof;   // optional cycle counters of CTA 0 (null: off)
-  unsigned long long* trace;  // optional [64][8] absolute cycle stamps of CTA 0's first K blocks
 };
 
 // mode 1: GEMM1 + SwiGLU + row amax; mode 2: GEMM2 + weighted combine.  Tiles of 128 rows x 256 weight rows.

@@ -81,7 +81,7 @@ typedef struct b200moe_ws_layout {
   uint64_t tok_rows;      /* int32[T][8]: packed row of (token,k), -1 if the expert is not local */
   uint64_t topk_ids;      /* int32[T][8]  (used by b200moe_run) */
   uint64_t topk_w;        /* float[T][8]  (used by b200moe_run) */
-  uint64_t trace;         /* uint64[2][64][8]: cycle stamps written when B200MOE_PROF is set */
+  uint64_t trace;         /* uint64[2][64][8]: room for cycle stamps of one-off probes (nothing in the library writes it) */
   uint64_t splitk_scratch; /* float[320][nt][128], nt = 16 up to 16 tokens, 64 up to 64, else 0: partial sums of slabs that the streaming GEMMs cut */
   uint64_t ep_segments;    /* 256 bytes: segment table and row count of b200moe_ep_local_experts (device-written) */
   int32_t m_cap;          /* capacity in packed rows (multiple of 128) */
