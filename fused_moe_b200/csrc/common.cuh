@@ -144,6 +144,12 @@ __device__ __forceinline__ void tma_load_4d(uint32_t smem_dst, const CUtensorMap
       ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
       : "memory");
 }
+// untiled bulk copy global -> shared (16-byte aligned, size a multiple of 16), counted on an mbarrier
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(smem_dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -292,6 +298,14 @@ __device__ __forceinline__ void st_global_v8(void* addr, const uint32_t (&v)[8])
                : "memory");
 }
 
+// SwiGLU of one pair (GEMM1's epilogues)
+__device__ __forceinline__ float silu_mul(float g, float u) {
+  float sig = __fdividef(1.0f, 1.0f + __expf(-u));   // approximate reciprocal: 2 ulp, far below e4m3 resolution
+  // The activations are stored as fp16: a product beyond its range saturates (the row then requantises to
+  // the largest e4m3 code) instead of becoming inf and, through an infinite row scale, NaN.
+  return fminf(fmaxf(g * (u * sig), -65504.0f), 65504.0f);
+}
+
 // four floats -> four e4m3 bytes (round to nearest even, saturating); byte order = element order
 __device__ __forceinline__ uint32_t pack4_e4m3(float a, float b, float c, float d) {
   uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(a, b), __NV_SATFINITE, __NV_E4M3);
@@ -325,10 +339,6 @@ __device__ __forceinline__ uint2 requant8(const uint4& raw, float scale, float i
 __device__ __forceinline__ void red_add_bf16x8(void* addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
   asm volatile("red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};" ::"l"(addr), "r"(a), "r"(b), "r"(c), "r"(d)
                : "memory");
-}
-
-__device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float c, float d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
 
 // out[g] = p[i + 32 g], g < 8, all eight loads in flight before the first conversion (a conversion behind each load makes

@@ -96,13 +96,6 @@ constexpr int kBarBytes = 256;
 constexpr int kSmemBytes = kStages * kStageBytes + kRingBytes + kPanelBytes + kBarBytes + 1024;   // + alignment slack
 constexpr int kTmemCols = 2 * kBN;
 
-__device__ __forceinline__ float silu_mul(float g, float u) {
-  float sig = __fdividef(1.0f, 1.0f + __expf(-u));   // approximate reciprocal: 2 ulp, far below e4m3 resolution
-  // The activations are stored as fp16: a product beyond its range saturates (the row then requantises to
-  // the largest e4m3 code) instead of becoming inf and, through an infinite row scale, NaN.
-  return fminf(fmaxf(g * (u * sig), -65504.0f), 65504.0f);
-}
-
 // acc[16 pairs] += scale * r[32] with packed fp32 FMAs (scalar FMAs measured the same)
 __device__ __forceinline__ void fma_chunk(float2* acc, const uint32_t (&r)[32], float sc) {
   const float2 s2 = make_float2(sc, sc);
@@ -111,12 +104,6 @@ __device__ __forceinline__ void fma_chunk(float2* acc, const uint32_t (&r)[32], 
     acc[j] = __ffma2_rn(make_float2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), s2, acc[j]);
 }
 
-// untiled bulk copy global -> shared (16-byte aligned, size a multiple of 16), counted on an mbarrier
-__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
 // Relaxed: what the counter publishes ("these TMEM columns sit in my registers") was completed by
 // tcgen05.wait::ld before this instruction; the tcgen05 fences on both sides order the tensor-memory accesses.
 __device__ __forceinline__ void red_add_smem(uint32_t addr, uint32_t v) {

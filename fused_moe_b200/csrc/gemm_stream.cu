@@ -73,19 +73,6 @@ template <int MODE, int NT> struct SCfg {
 };
 static_assert(kGroup == 2, "the promotion loop below reads two K blocks per hand-off");
 
-__device__ __forceinline__ float silu_mul(float g, float u) {
-  float sig = __fdividef(1.0f, 1.0f + __expf(-u));
-  // The activations are stored as fp16: a product beyond its range saturates (the row then requantises to
-  // the largest e4m3 code) instead of becoming inf and, through an infinite row scale, NaN.
-  return fminf(fmaxf(g * (u * sig), -65504.0f), 65504.0f);
-}
-
-__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-
 // 32 lanes x 16 consecutive fp32 columns, and waits that name the loaded registers
 __device__ __forceinline__ void tmem_ld_16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(

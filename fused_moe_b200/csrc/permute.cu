@@ -202,7 +202,7 @@ cudaError_t launch_permute(const Workspace& ws, const int32_t* ids, long long id
   }
   if (n_chunks > 0) {
     if (!placed) {
-        err = launch_chained(place_kernel, dim3(n_chunks), dim3(1024), 0, stream, ws, ids, ids_stride, w, w_stride, T,
+      err = launch_chained(place_kernel, dim3(n_chunks), dim3(1024), 0, stream, ws, ids, ids_stride, w, w_stride, T,
                            local_off, e_local, n_rows_dev);
       if (err != cudaSuccess) return err;
     }
