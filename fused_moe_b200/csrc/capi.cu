@@ -146,7 +146,11 @@ constexpr int kZeroInGemmExperts = 4;
 constexpr int kDirectRowsMaxTokens = 8;   // largest call whose decode GEMM1 reads the caller's rows in place
 
 // Decode-size calls (up to 16 tokens) requantise inside GEMM1 (B200MOE_DECODE=0 turns that off, B200MOE_DECODE=64
-// extends it to 64 tokens).  Returns the token tile of the streaming kernels for such a call, or 0.
+// extends it to 64 tokens).  Above 16 tokens the pass of its own is the default: the CTA that stores an expert's last slab
+// turns up to 64 rows into codes alone, which takes longer than the launch it saves once experts hold more than a few rows.  us a
+// call, pass / inside GEMM1 (32 experts): 17 tokens, 5 active experts 81.9 / 79.9, 8 active 98.3 / 102.4; 56 tokens, 14 active
+// 147.5 / 149.5, 17 active 163.9 / 170.0; a Zipf load 17 tokens 108.5 / 120.8, 32 tokens 112.6 / 137.2, 64 tokens 116.8 / 170.0.
+// Returns the token tile of the streaming kernels for such a call, or 0.
 int decode_tile(int T) {
   static const bool decode_on = [] {
     const char* v = getenv("B200MOE_DECODE");
@@ -162,9 +166,11 @@ int decode_tile(int T) {
 // Calls above the decode sizes and up to this many tokens take the weight-streaming GEMMs if few enough experts are local.
 // The 128 x 256 tiles of the grouped kernel come in whole waves of SMs: with some ten to twenty active experts (two waves
 // of GEMM1 items) the second is mostly idle, with more than a hundred it does not matter and the grouped kernel's larger
-// boxes win (32 experts: 20 tokens 133 -> 117 us with 12 active, 56 tokens 131 -> 115 with 10 and 160 -> 154 with 18, 64
-// tokens on a Zipf load, every expert with some 60 rows, 103 -> 107; 64 tokens over 64 experts 265 -> 250, over 256
-// 915 -> 945).  B200MOE_STREAM=0: never.
+// boxes win.  us a call, grouped / streaming: 32 experts, 17 tokens on 8 active 104.5 / 98.3, 20 on 10 137.2 / 116.8, 33 on 17
+// 172.1 / 163.9, 56 on 14 153.7 / 147.5, 64 on 19 204.8 / 180.3; 64 experts, 33 tokens on 28 270.4 / 239.6, 64 on 34 288.8 /
+// 278.6; 256 experts, 64 tokens 915 / 945.  A Zipf load, all rows on nine experts: 17 tokens 110.7 / 108.5, 32 tokens 114.8 /
+// 112.6, 40 tokens 114.7 / 114.7, 48 to 60 tokens 114.8 / 116.7, 64 tokens 116.7 / 116.8.  (Between 64 and 256 experts nothing was
+// measured; they keep the grouped kernels.)  B200MOE_STREAM=0: never.
 constexpr int kStreamMaxTokens = 64;
 constexpr int kStreamMaxExperts = 64;
 // Returns the most token rows of a tile (an expert of a call of at most 64 tokens has no more), or 0 for the grouped kernels.

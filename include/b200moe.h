@@ -150,6 +150,9 @@ B200MOE_API int b200moe_count(const int32_t* topk_ids, int64_t ids_row_stride, i
  * filled by b200moe_route or b200moe_count for the same ids on the same stream.  The call zeroes the T
  * output rows itself and GEMM2's epilogue adds every (token, expert) row into its token's row in bf16
  * (no combine pass; the sum order follows tile completion, so two runs agree to a few bf16 steps).
+ * At up to 64 tokens the K range of a weight slab may be summed in pieces whose bounds follow from the call's
+ * number of active experts, so a token's row can differ in the last bits with the tokens beside it: an activation on a
+ * rounding boundary may take the neighbouring e4m3 code.  Larger calls sum every K range in one fixed order.
  * Replaces `fused_dispatch`, `fused_gather_hidden_scales`, `moe_blockwise_grouped_mm_v2`
  * (x2), `swiglu_fp8_requant*`, `weighted_scatter` / `reduce_scatter_unweighted_fused`
  * (moe_fused.cu:131-542, 736-1150; moe_gemm.cu:527-654).

@@ -6,7 +6,7 @@ tokens against the oracle.
 A token's output row is the sum of its (at most eight) expert rows, each rounded to bf16 and added
 by GEMM2's epilogue with a bf16 `red.global.add` in whatever order the tiles finish - the reference's
 `out[t] += bf16(G2 * w)` on a bf16 tensor, in a free order.  Everything before that sum is
-order-deterministic, so two runs differ by the rounding of at most eight bf16 additions:
+order-deterministic for one and the same call, so two runs differ by the rounding of at most eight bf16 additions:
 a few bf16 steps of the largest partial sum.  `_same_up_to_sum_order` asserts exactly that."""
 import numpy as np
 import pytest
@@ -54,8 +54,8 @@ def test_repeat_differs_by_fp32_sum_order_only_at_4096_tokens(full_weights_gpu):
 
 
 def test_token_permutation_permutes_the_output_rows(full_weights_gpu):
-    """A token's result depends on no other token: same K order and same promotion order whatever
-    packed row it lands in; only the order of the final fp32 additions is free."""
+    """A token's result depends on no other token at these sizes: the 128 x 256 tiles sum K in the same order
+    whatever packed row it lands in; only the order of the final bf16 additions is free."""
     dev = torch.device("cuda", 0)
     bias = synth.make_bias(0).to(dev)
     lg, hq, hsc = _tokens(4096, 0, dev)
@@ -70,10 +70,11 @@ def test_subset_of_tokens_gives_the_same_rows(full_weights_gpu):
     bias = synth.make_bias(0).to(dev)
     lg, hq, hsc = _tokens(4096, 0, dev)
     base = _run(lg, bias, hq, hsc, full_weights_gpu)
-    # 64 tokens: same kernels (128-row tiles), so the same values up to the order of the final sums
+    # 64 tokens: the streaming kernels, which sum a slab's K range in pieces: beside the order of the final sums an
+    # activation may take the neighbouring e4m3 code, one of 2048 terms of an output by a sixteenth of its size
     sub = _run(lg[:64].contiguous(), bias, hq[:64].contiguous(), hsc[:, :64].contiguous(), full_weights_gpu)
     _same_up_to_sum_order(sub, base[:64])
-    # 16 tokens: the swapped-operand decode kernels; same arithmetic order, compared at the layer's tolerance
+    # 16 tokens: the streaming kernels with requantisation inside, compared at the layer's tolerance
     sub = _run(lg[:16].contiguous(), bias, hq[:16].contiguous(), hsc[:, :16].contiguous(), full_weights_gpu)
     frac_all, frac_nz, max_abs = synth.check_close(sub, base[:16].cpu())
     assert frac_all >= 0.999 and frac_nz >= 0.999, (frac_all, frac_nz, max_abs)
