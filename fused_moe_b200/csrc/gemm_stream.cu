@@ -633,8 +633,9 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
             }
             transpose8(v, lane);
             const int t = t0 + (lane & 7);
-            const int tok = t < cnt ? p.row_token[row0 + t] : -1;
-            if (tok >= 0) {
+            if (t < cnt) {
+              // the three loads together: behind the check of the token the other two would wait for it
+              const int tok = p.row_token[row0 + t];
               const float rs = p.row_scale[row0 + t] * p.row_weight[row0 + t];
               uint32_t wv[4];
 #pragma unroll
@@ -642,7 +643,7 @@ stream_gemm_kernel(const __grid_constant__ StreamParams sp) {
                 __nv_bfloat162 b2 = __floats2bfloat162_rn(v[2 * j] * rs, v[2 * j + 1] * rs);
                 wv[j] = *reinterpret_cast<uint32_t*>(&b2);
               }
-              red_add_bf16x8(dst + (size_t)tok * p.out_stride, wv[0], wv[1], wv[2], wv[3]);
+              if (tok >= 0) red_add_bf16x8(dst + (size_t)tok * p.out_stride, wv[0], wv[1], wv[2], wv[3]);
             }
           }
         }
