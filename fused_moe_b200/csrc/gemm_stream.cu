@@ -50,7 +50,7 @@ template <int MODE, int NT> struct SCfg {
   static constexpr int kStageBytes = kGroup * (kWBytes + kTokBytes);  // [group][128 weight rows], [group][NT token rows]
   static constexpr int kStages = NT <= 16 ? 5 : 4;
   static constexpr int kIssuers = 2;
-  static constexpr int kProducers = NT <= 16 ? kStages : 2;   // (12 warps in all: a 13th costs every thread 40 registers)
+  static constexpr int kProducers = NT <= 16 ? kStages : 2;   // (12 warps in all: a 13th costs every thread 40 registers; at 168 <1, 64> spills 16 bytes)
   // The roles wait by parity, so nobody may wait for a phase while the one before last is still open.  A producer owns its
   // stages.  The issuers take turns on an odd number of stages; an issuer waits for its accumulators first, i.e. until group
   // it - kAccs has been promoted, and that has to cover the stage's previous use, group it - kStages.
